@@ -82,20 +82,13 @@ def _side(rng, lo, hi):
     return int(round(math.exp(rng.uniform(math.log(lo), math.log(hi)))))
 
 
-def _rows(h):
-    """Heights of 16 k + 1 rows are left out: versions of the library before the
-    tiles' reflections were bounded read outside shared memory there, and a
-    comparison with one of them must not fault the GPU."""
-    return h + 1 if h % 16 == 1 else h
-
-
 def draw(rng):
     kind = rng.choice(["frame"] * 6 + ["batch", "deposit", "lit", "relief", "resolve"])
     if kind == "frame":
         field = rng.choice(["blobs", "blobs", "drips", "drips", "pours"])
         side = _side(rng, 64, 1100 if field == "pours" else 3600)
         a = math.sqrt(rng.uniform(0.5, 2.0))
-        w, h = max(48, int(side * a)), _rows(max(48, int(side / a)))
+        w, h = max(48, int(side * a)), max(48, int(side / a))
         per = {"blobs": CELLS_PER_BLOB, "drips": CELLS_PER_LINE, "pours": CELLS_PER_POUR}[field]
         count = max(3, int(w * h / per * rng.uniform(0.5, 2.0)))
         drive = rng.choice(["adaptive", "app"]) if field == "pours" else rng.choice(["fixed", "adaptive"])
@@ -106,7 +99,7 @@ def draw(rng):
         return dict(kind=kind, films=rng.randint(3, 24), lo=lo, hi=int(lo * rng.uniform(1.5, 3.0)),
                     prec=rng.choice(["ref", "fp32", "bf16"]))
     side = _side(rng, 300, 2048)
-    w, h = side, _rows(max(64, int(side * rng.uniform(0.6, 1.0))))
+    w, h = side, max(64, int(side * rng.uniform(0.6, 1.0)))
     if kind == "deposit":
         return dict(kind=kind, w=w, h=h, strokes=_side(rng, 4, 1024), prec=rng.choice(["ref", "fp32", "bf16"]))
     vw = _side(rng, 160, 1920)
@@ -316,7 +309,7 @@ def _batch_sizes(c):
     out = []
     for k in range(n):
         side = c["lo"] * (c["hi"] / c["lo"]) ** (k / max(n - 1, 1))
-        out.append(_rows(int(side) + 1) if k % 5 == 4 else max(48, int(round(side / 16.0)) * 16))
+        out.append(int(side) + 1 if k % 5 == 4 else max(48, int(round(side / 16.0)) * 16))
     return out
 
 
