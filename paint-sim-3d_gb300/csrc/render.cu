@@ -22,7 +22,8 @@
 // decide the comparison it feeds (BUMP_LO, BUMP_HI): 1920x1080 over bare and
 // painted canvas 2620 -> 1450 us (2476 with the split alone, 2234 with the
 // bounds, then in step 1752 at 32 x 32 threads a block, 1550 at 16 x 32, 1450
-// with five more meeting points after the bisection).
+// with five more meeting points after the bisection; 1496 now that finished
+// pixels and lanes outside the picture pass the meeting points too).
 //
 // Every function follows the shader's f32 arithmetic in its order of
 // operations; this file is compiled without multiply-add contraction, so the
@@ -476,14 +477,12 @@ __device__ __noinline__ float micro(const R& X, float2 p, const Detail& d) {
   }
   return z;
 }
-// micro() where bare_weave holds.
-template <class R>
-__device__ __forceinline__ float canvas_bump_full(const R& X, float2 p, const Detail& d) {
-  return micro(X, p, d);
-}
 // Keeps the block's warps in one stretch of code: they fetch a step's
-// instructions once instead of each at its own time.  Every thread that has not
-// returned from the kernel passes the same sequence of these.
+// instructions once instead of each at its own time.  Called in uniform control
+// flow only: every thread of the block passes the same sequence of these, those
+// outside the picture and those whose pixel is finished too (a lane that left
+// early would wait for its warp to reconverge while the warp's others wait at
+// the barrier).
 __device__ __forceinline__ void in_step() { __syncthreads(); }
 template <class R>
 __device__ __noinline__ float2 micro_slope(const R& X, float2 p, const Detail& d) {
@@ -820,8 +819,9 @@ __device__ __noinline__ float shadow_at(const R& X, float2 p, float z0, float3 l
   }
   return sh;
 }
+// Every thread of the block calls it; only those with `live` evaluate samples.
 template <class R>
-__device__ __noinline__ float ambient_occlusion(const R& X, float2 p, float z0, const Detail& d) {
+__device__ __noinline__ float ambient_occlusion(const R& X, bool live, float2 p, float z0, const Detail& d) {
   const float step = X.cam.canvas[2] * 2.0f;
   const bool bare = bare_weave(X, d);
   float open = 0.0f;
@@ -833,13 +833,14 @@ __device__ __noinline__ float ambient_occlusion(const R& X, float2 p, float z0, 
 #pragma unroll 1
     for (int i = 1; i <= AO_STEPS; ++i) {
       in_step();
+      if (!live) continue;
       const float dist = (float)i * step;
       const float2 q = p + dir * dist;
       if (bare) {
         // a sample that cannot rise above the horizon, whatever the weave adds
         const float base = surf_bilinear(X, q);
         if (base + BUMP_HI - z0 <= horizon * dist) continue;
-        const float rise = base + canvas_bump_full(X, q, d) - z0;
+        const float rise = base + micro(X, q, d) - z0;
         horizon = fmaxf(horizon, rise / dist);
       } else {
         const float rise = surf_hit(X, q, d) - z0;
@@ -977,53 +978,77 @@ __device__ float3 mat_ray(const cf_render_cam& cam, float x, float y, float z) {
 }
 
 // ---- the fragment (render.wgsl:985-1116)
-template <class R>
-__device__ float4 fs(const R& X, float2 ndc_in) {
-  const float2 ndc = ndc_in + v2(X.cam.jitter[0], X.cam.jitter[1]);
-  float3 a = mat_ray(X.cam, ndc.x, ndc.y, 0.0f);
-  float3 dir = nrm3(mat_ray(X.cam, ndc.x, ndc.y, 1.0f) - a);
-  if (X.cam.ortho[0] > 0.5f) {
-    const float2 pxy = (ndc * 0.5f + v2(0.5f, 0.5f)) * v2(X.cam.canvas[0], X.cam.canvas[1]);
-    a = v3(pxy.x, pxy.y, 1.0f);
-    dir = v3(0.0f, 0.0f, -1.0f);
-  } else if (X.cam.lens[3] > 0.5f) {
-    const float3 br = v3(X.cam.basis_r[0], X.cam.basis_r[1], X.cam.basis_r[2]);
-    const float3 bu = v3(X.cam.basis_u[0], X.cam.basis_u[1], X.cam.basis_u[2]);
-    const float3 fwd = cross3(bu, br);
-    const float fd = X.cam.lens[2] / fmaxf(dot3(dir, fwd), 1e-3f);
-    const float3 fp = a + dir * fd;
-    a = a + br * X.cam.lens[0] + bu * X.cam.lens[1];
-    dir = nrm3(fp - a);
-  }
-  const float3 bg = mix3(v3(X.cam.ground[0], X.cam.ground[1], X.cam.ground[2]), v3(X.cam.sky[0], X.cam.sky[1], X.cam.sky[2]),
-                         clampf(dir.z * 0.5f + 0.5f, 0.0f, 1.0f));
-  if (fabsf(dir.z) < 1e-5f) { const float3 c = to_srgb(tonemap(bg)); return make_float4(c.x, c.y, c.z, 1.0f); }
-  const float t1 = -a.z / dir.z;
-  if (t1 < 0.0f) { const float3 c = to_srgb(tonemap(bg)); return make_float4(c.x, c.y, c.z, 1.0f); }
-  const float top = X.cam.canvas[3];
-  float t0 = 0.0f;
-  if (a.z > top) t0 = (top - a.z) / dir.z;
-  const float span = fmaxf(t1 - t0, 0.0f);
-  const float horiz = span * len2(v2(dir.x, dir.y));
-  const int nsteps = min(max((int)ceilf(horiz / X.cam.canvas[2]), 1), 96);
-  const float step = span / (float)nsteps;
-  float ta = t0, tb = t1;
-  bool found = false;
-#pragma unroll 1
-  for (int k = 1; k <= nsteps; ++k) {
-    const float tk = t0 + (float)k * step;
-    const float3 q = a + dir * tk;
-    if (q.z <= surf_march(X, v2(q.x, q.y))) {
-      tb = tk;
-      found = true;
-      break;
+// Where a fragment goes: pixel o of the outputs that are wanted.
+struct Target {
+  float4* f32;
+  uint32_t* rgba8;
+  size_t o;
+  __device__ __noinline__ void put(float3 c) const {
+    if (f32) f32[o] = make_float4(c.x, c.y, c.z, 1.0f);
+    if (rgba8) {
+      auto q = [](float x) { return (uint32_t)fminf(fmaxf(x * 255.0f + 0.5f, 0.0f), 255.0f); };
+      rgba8[o] = q(c.x) | (q(c.y) << 8) | (q(c.z) << 16) | (q(1.0f) << 24);
     }
-    ta = tk;
   }
-  float t = t1;
-  const float3 qb = a + dir * tb;
-  const Detail detail = detail_params(X, v2(qb.x, qb.y));
-  const bool weave_only = bare_weave(X, detail);
+};
+// Every thread of the block calls it (in_step); a thread without `live` has no
+// pixel, or has put it already.
+template <class R>
+__device__ __forceinline__ void fs(const R& X, bool live, float2 ndc_in, const Target& out) {
+  float3 a = v3(0.0f, 0.0f, 0.0f), dir = a;
+  float ta = 0.0f, tb = 0.0f, t1 = 0.0f;
+  bool found = false, weave_only = false;
+  Detail detail = {};
+  if (live) {
+    const float2 ndc = ndc_in + v2(X.cam.jitter[0], X.cam.jitter[1]);
+    a = mat_ray(X.cam, ndc.x, ndc.y, 0.0f);
+    dir = nrm3(mat_ray(X.cam, ndc.x, ndc.y, 1.0f) - a);
+    if (X.cam.ortho[0] > 0.5f) {
+      const float2 pxy = (ndc * 0.5f + v2(0.5f, 0.5f)) * v2(X.cam.canvas[0], X.cam.canvas[1]);
+      a = v3(pxy.x, pxy.y, 1.0f);
+      dir = v3(0.0f, 0.0f, -1.0f);
+    } else if (X.cam.lens[3] > 0.5f) {
+      const float3 br = v3(X.cam.basis_r[0], X.cam.basis_r[1], X.cam.basis_r[2]);
+      const float3 bu = v3(X.cam.basis_u[0], X.cam.basis_u[1], X.cam.basis_u[2]);
+      const float3 fwd = cross3(bu, br);
+      const float fd = X.cam.lens[2] / fmaxf(dot3(dir, fwd), 1e-3f);
+      const float3 fp = a + dir * fd;
+      a = a + br * X.cam.lens[0] + bu * X.cam.lens[1];
+      dir = nrm3(fp - a);
+    }
+    t1 = -a.z / dir.z;
+    if (fabsf(dir.z) < 1e-5f || t1 < 0.0f) {
+      const float3 bg = mix3(v3(X.cam.ground[0], X.cam.ground[1], X.cam.ground[2]),
+                             v3(X.cam.sky[0], X.cam.sky[1], X.cam.sky[2]), clampf(dir.z * 0.5f + 0.5f, 0.0f, 1.0f));
+      out.put(to_srgb(tonemap(bg)));
+      live = false;
+    }
+  }
+  if (live) {
+    const float top = X.cam.canvas[3];
+    float t0 = 0.0f;
+    if (a.z > top) t0 = (top - a.z) / dir.z;
+    const float span = fmaxf(t1 - t0, 0.0f);
+    const float horiz = span * len2(v2(dir.x, dir.y));
+    const int nsteps = min(max((int)ceilf(horiz / X.cam.canvas[2]), 1), 96);
+    const float step = span / (float)nsteps;
+    ta = t0;
+    tb = t1;
+#pragma unroll 1
+    for (int k = 1; k <= nsteps; ++k) {
+      const float tk = t0 + (float)k * step;
+      const float3 q = a + dir * tk;
+      if (q.z <= surf_march(X, v2(q.x, q.y))) {
+        tb = tk;
+        found = true;
+        break;
+      }
+      ta = tk;
+    }
+    const float3 qb = a + dir * tb;
+    detail = detail_params(X, v2(qb.x, qb.y));
+    weave_only = bare_weave(X, detail);
+  }
 #pragma unroll 1
   for (int r = 0; r < 8; ++r) {
     in_step();
@@ -1034,101 +1059,112 @@ __device__ float4 fs(const R& X, float2 ndc_in) {
     const float base = weave_only ? surf_bilinear(X, v2(q.x, q.y)) : 0.0f;
     if (weave_only && q.z <= base + BUMP_LO) under = true;       // whatever the weave
     else if (weave_only && q.z > base + BUMP_HI) under = false;  // adds there
-    else if (weave_only) under = q.z <= base + canvas_bump_full(X, v2(q.x, q.y), detail);
+    else if (weave_only) under = q.z <= base + micro(X, v2(q.x, q.y), detail);
     else under = q.z <= surf_hit(X, v2(q.x, q.y), detail);
     if (under) tb = tm;
     else ta = tm;
   }
-  if (found) t = tb;
-  const float3 hit = a + dir * t;
+  const float3 hit = a + dir * (found ? tb : t1);
   const float2 p = v2(hit.x, hit.y);
   const float W = X.cam.canvas[0], H = X.cam.canvas[1];
-  if (p.x < 0.0f || p.y < 0.0f || p.x > W || p.y > H) {
-    const float3 c = to_srgb(tonemap(floor_color()));
-    return make_float4(c.x, c.y, c.z, 1.0f);
-  }
   const float3 v = -dir;
   const float3 l = nrm3(v3(X.cam.light[0], X.cam.light[1], X.cam.light[2]));
-  if (!near_paint(X, p) && !X.beauty()) {
-    const float4 cs = color_sharp(X, p);
-    const float3 c = to_srgb(tonemap(lit(X, normal_bilinear(X, p), v, l, 1.0f, 1.0f, rgb(cs), cs.w, 0.0f, 0.0f, 0.0f,
-                                         v2(1.0f, 0.0f), 1.0f)));
-    return make_float4(c.x, c.y, c.z, 1.0f);
+  if (live) {
+    if (p.x < 0.0f || p.y < 0.0f || p.x > W || p.y > H) {
+      out.put(to_srgb(tonemap(floor_color())));
+      live = false;
+    } else if (!X.beauty() && !near_paint(X, p)) {
+      const float4 cs = color_sharp(X, p);
+      out.put(to_srgb(tonemap(lit(X, normal_bilinear(X, p), v, l, 1.0f, 1.0f, rgb(cs), cs.w, 0.0f, 0.0f, 0.0f,
+                                  v2(1.0f, 0.0f), 1.0f))));
+      live = false;
+    }
+  }
+  if (!__syncthreads_or(live)) return;  // the block's pixels are finished
+  float2 ms = v2(0.0f, 0.0f), pc = p;
+  float3 n = v3(0.0f, 0.0f, 1.0f);
+  if (live) {
+    ms = micro_slope(X, p, detail);
+    n = normal_from_slope(base_slope(X, p) + ms);
+    const float slope = len2(v2(n.x, n.y)) / fmaxf(n.z, 1e-3f);
+    if (slope > 0.4f) {
+      const float2 up = nrm2(v2(-n.x, -n.y));
+      pc = p + up * X.cam.canvas[2] * (0.5f + clampf(slope, 0.0f, 3.0f) * 0.5f);
+      pc = v2(clampf(pc.x, 0.0f, W), clampf(pc.y, 0.0f, H));
+    }
   }
   in_step();
-  const float2 ms = micro_slope(X, p, detail);
-  const float3 n = normal_from_slope(base_slope(X, p) + ms);
-  const float slope = len2(v2(n.x, n.y)) / fmaxf(n.z, 1e-3f);
-  float2 pc = p;
-  if (slope > 0.4f) {
-    const float2 up = nrm2(v2(-n.x, -n.y));
-    pc = p + up * X.cam.canvas[2] * (0.5f + clampf(slope, 0.0f, 3.0f) * 0.5f);
-    pc = v2(clampf(pc.x, 0.0f, W), clampf(pc.y, 0.0f, H));
+  float4 col = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  float thin = 0.0f, rough = 0.0f, z0 = 0.0f, sh = 1.0f;
+  if (live) {
+    const float2 pcw = cwarp(X, pc, detail);
+    col = color_sharp(X, pcw);
+    if (X.beauty() && detail.thickness > 0.02e-3f) {
+      const float3 m = marble(X, pcw, rgb(col), detail);
+      col = make_float4(m.x, m.y, m.z, col.w);
+    }
+    thin = 0.3f * (1.0f - sstep(0.0f, THIN_FILM_MATTE, detail.thickness)) * sstep(0.0f, 1e-5f, detail.thickness);
+    rough = clampf(col.w + 0.3f * len2(ms) + thin, 0.03f, 0.95f);
+    if (X.beauty()) {
+      const float paint_cover = sstep(0.0f, 0.08e-3f, detail.thickness);
+      const float gloss = DRY_GLOSS_FLOOR + (col.w - DRY_GLOSS_FLOOR) * DRY_GLOSS_SCALE;
+      const float patchy = 0.75f + 0.5f * (0.5f + 0.5f * fbm(p / 2.5e-3f + v2(6.1f, 2.4f), 3));
+      rough = clampf(mixf(col.w, gloss * patchy, paint_cover) + thin, 0.03f, 0.95f);
+    }
+    z0 = surf_hit(X, p, detail);
   }
   in_step();
-  const float2 pcw = cwarp(X, pc, detail);
-  float4 col = color_sharp(X, pcw);
-  if (X.beauty() && detail.thickness > 0.02e-3f) {
-    const float3 m = marble(X, pcw, rgb(col), detail);
-    col = make_float4(m.x, m.y, m.z, col.w);
-  }
-  const float thin = 0.3f * (1.0f - sstep(0.0f, THIN_FILM_MATTE, detail.thickness)) * sstep(0.0f, 1e-5f, detail.thickness);
-  float rough = clampf(col.w + 0.3f * len2(ms) + thin, 0.03f, 0.95f);
-  if (X.beauty()) {
-    const float paint_cover = sstep(0.0f, 0.08e-3f, detail.thickness);
-    const float gloss = DRY_GLOSS_FLOOR + (col.w - DRY_GLOSS_FLOOR) * DRY_GLOSS_SCALE;
-    const float patchy = 0.75f + 0.5f * (0.5f + 0.5f * fbm(p / 2.5e-3f + v2(6.1f, 2.4f), 3));
-    rough = clampf(mixf(col.w, gloss * patchy, paint_cover) + thin, 0.03f, 0.95f);
-  }
-  const float z0 = surf_hit(X, p, detail);
+  if (live) sh = shadow_at(X, p, z0, l);
   in_step();
-  const float sh = shadow_at(X, p, z0, l);
-  in_step();
-  const float ao = ambient_occlusion(X, p, z0, detail);
+  const float ao = ambient_occlusion(X, live, p, z0, detail);
   float3 albedo = rgb(col);
-  const float painted = sstep(0.0f, 0.08e-3f, detail.thickness);
-  if (painted > 0.0f) {
-    const float g = granulation(p);
-    albedo = albedo * (1.0f + 0.045f * g * painted);
-    const float rim = edge_factor(X, p);
-    albedo = albedo * (1.0f - 0.10f * rim * painted);
+  float rough_s = 0.0f, coat = 0.0f, aniso = 0.0f, falloff = 1.0f;
+  if (live) {
+    const float painted = sstep(0.0f, 0.08e-3f, detail.thickness);
+    if (painted > 0.0f) {
+      const float g = granulation(p);
+      albedo = albedo * (1.0f + 0.045f * g * painted);
+      const float rim = edge_factor(X, p);
+      albedo = albedo * (1.0f - 0.10f * rim * painted);
+    }
+    if (X.beauty() && painted > 0.0f) {
+      const float2 sc = streak_coords(p, detail.dir);
+      const float tool = clampf(detail.brush + detail.knife, 0.0f, 1.0f);
+      const float st = fbm_filtered(X, v2(sc.x, sc.y / 25.0f), 0.09e-3f, 4);
+      albedo = albedo * (1.0f + 0.16f * st * (0.3f + 0.7f * tool) * painted);
+      const float cl = fbm_filtered(X, v2(sc.x, sc.y / CLUMP_ELONGATION), CLUMP_WIDTH, 3);
+      albedo = albedo * (1.0f + 0.10f * cl * tool * painted);
+      const float thin_paint = 1.0f - sstep(0.03e-3f, 0.25e-3f, detail.thickness);
+      const float3 wv = weave(p);
+      albedo = albedo * (1.0f + 0.22f * thin_paint * (wv.x - 0.55f) * painted);
+    }
+    const float bare = 1.0f - sstep(0.0f, 0.15e-3f, detail.thickness);
+    if (bare > 0.0f) albedo = mix3(albedo, canvas_albedo(p, albedo), bare);
+    if (X.beauty() && painted > 0.0f) {
+      const float3 hue = v3(fbm(p / 6e-3f + v2(1.3f, 5.1f), 3), fbm(p / 6e-3f + v2(7.7f, 2.2f), 3),
+                            fbm(p / 6e-3f + v2(4.4f, 9.9f), 3));
+      const float tone = fbm(p / 2.2e-3f + v2(3.3f, 0.7f), 4);
+      albedo = albedo * ((v3(1.0f, 1.0f, 1.0f) + PAINT_HUE_DRIFT * hue) * (1.0f + PAINT_TONE_DRIFT * tone * painted));
+    }
+    const float2 sp = specks(p);
+    albedo = mix3(albedo, v3(0.85f, 0.83f, 0.8f), 0.7f * sp.x * (0.4f + 0.6f * bare));
+    albedo = albedo * (1.0f - 0.6f * sp.y);
+    const float rough_var = 1.0f + 0.18f * vnoise(p / 0.45e-3f + v2(3.0f, 8.0f)) * painted;
+    rough_s = clampf(rough * rough_var, 0.03f, 0.95f);
+    const float wetness = wet_bilinear(X, p);
+    coat = sstep(0.02e-3f, 0.25e-3f, wetness) * (1.0f - 0.7f * detail.cure) * (1.0f - thin / 0.3f);
+    aniso = clampf(0.7f * detail.brush + 0.5f * detail.knife, 0.0f, 0.8f) * sstep(0.0f, 0.15e-3f, detail.thickness);
+    if (X.beauty()) falloff = lamp_falloff(X, p);
   }
-  if (X.beauty() && painted > 0.0f) {
-    const float2 sc = streak_coords(p, detail.dir);
-    const float tool = clampf(detail.brush + detail.knife, 0.0f, 1.0f);
-    const float st = fbm_filtered(X, v2(sc.x, sc.y / 25.0f), 0.09e-3f, 4);
-    albedo = albedo * (1.0f + 0.16f * st * (0.3f + 0.7f * tool) * painted);
-    const float cl = fbm_filtered(X, v2(sc.x, sc.y / CLUMP_ELONGATION), CLUMP_WIDTH, 3);
-    albedo = albedo * (1.0f + 0.10f * cl * tool * painted);
-    const float thin_paint = 1.0f - sstep(0.03e-3f, 0.25e-3f, detail.thickness);
-    const float3 wv = weave(p);
-    albedo = albedo * (1.0f + 0.22f * thin_paint * (wv.x - 0.55f) * painted);
-  }
-  const float bare = 1.0f - sstep(0.0f, 0.15e-3f, detail.thickness);
-  if (bare > 0.0f) albedo = mix3(albedo, canvas_albedo(p, albedo), bare);
-  if (X.beauty() && painted > 0.0f) {
-    const float3 hue = v3(fbm(p / 6e-3f + v2(1.3f, 5.1f), 3), fbm(p / 6e-3f + v2(7.7f, 2.2f), 3),
-                          fbm(p / 6e-3f + v2(4.4f, 9.9f), 3));
-    const float tone = fbm(p / 2.2e-3f + v2(3.3f, 0.7f), 4);
-    albedo = albedo * ((v3(1.0f, 1.0f, 1.0f) + PAINT_HUE_DRIFT * hue) * (1.0f + PAINT_TONE_DRIFT * tone * painted));
-  }
-  const float2 sp = specks(p);
-  albedo = mix3(albedo, v3(0.85f, 0.83f, 0.8f), 0.7f * sp.x * (0.4f + 0.6f * bare));
-  albedo = albedo * (1.0f - 0.6f * sp.y);
-  const float rough_var = 1.0f + 0.18f * vnoise(p / 0.45e-3f + v2(3.0f, 8.0f)) * painted;
-  const float rough_s = clampf(rough * rough_var, 0.03f, 0.95f);
-  const float wetness = wet_bilinear(X, p);
-  const float coat = sstep(0.02e-3f, 0.25e-3f, wetness) * (1.0f - 0.7f * detail.cure) * (1.0f - thin / 0.3f);
-  const float aniso = clampf(0.7f * detail.brush + 0.5f * detail.knife, 0.0f, 0.8f) * sstep(0.0f, 0.15e-3f, detail.thickness);
-  const float falloff = X.beauty() ? lamp_falloff(X, p) : 1.0f;
   in_step();
+  if (!live) return;
   const float3 c = lit(X, n, v, l, sh, ao, albedo, rough_s, detail.cure, coat, aniso, detail.dir, falloff);
   if (X.beauty()) {
     auto fc = [](float x) { return x != x ? 0.0f : fminf(x, FIREFLY_CLAMP); };
-    return make_float4(fc(c.x), fc(c.y), fc(c.z), 1.0f);
+    out.put(v3(fc(c.x), fc(c.y), fc(c.z)));
+  } else {
+    out.put(to_srgb(tonemap(c)));
   }
-  const float3 o = to_srgb(tonemap(c));
-  return make_float4(o.x, o.y, o.z, 1.0f);
 }
 
 // Blocks of LIT_W x ROWS pixels, 32 warps an SM.  A tall block shares each fetch
@@ -1145,15 +1181,9 @@ __global__ void __launch_bounds__(LIT_W* ROWS, 1024u / (LIT_W * ROWS))
     k_render_lit(const __grid_constant__ Bindings<BEAUTY> X, uint32_t width, uint32_t height, float4* out_f32,
                  uint32_t* out_rgba8) {
   const uint32_t px = blockIdx.x * LIT_W + threadIdx.x, py = blockIdx.y * ROWS + threadIdx.y;
-  if (px >= width || py >= height) return;
+  const bool live = px < width && py < height;
   const float2 ndc = v2(2.0f * ((float)px + 0.5f) / (float)width - 1.0f, 1.0f - 2.0f * ((float)py + 0.5f) / (float)height);
-  const float4 c = fs(X, ndc);
-  const size_t o = (size_t)py * width + px;
-  if (out_f32) out_f32[o] = c;
-  if (out_rgba8) {
-    auto q = [](float x) { return (uint32_t)fminf(fmaxf(x * 255.0f + 0.5f, 0.0f), 255.0f); };
-    out_rgba8[o] = q(c.x) | (q(c.y) << 8) | (q(c.z) << 16) | (q(c.w) << 24);
-  }
+  fs(X, live, ndc, Target{out_f32, out_rgba8, live ? (size_t)py * width + px : 0u});
 }
 
 }  // namespace
