@@ -634,12 +634,14 @@ __global__ void __launch_bounds__(256 * GROUPS, PER_SM)
   SolveGroup& G = reinterpret_cast<SolveGroup*>(solve_smem)[threadIdx.z];
   const int li = (int)(threadIdx.y * 16u + threadIdx.x), lane = li & 31;
   constexpr uint32_t ON = ACTIVE | 1u;  // an active tile that holds paint
-  bool any = false;
-  for (uint32_t f = 0; f < nfilms; ++f) any = any || step < (ONE ? only : films[f]).P->implicit_steps;
-  if (!any) return;  // no film takes this step: the same for every block
+  // the blocks meet at the first film that takes the step (a film without
+  // implicit steps has no CgState)
+  uint32_t first = 0;
+  while (first < nfilms && step >= (ONE ? only : films[first]).P->implicit_steps) ++first;
+  if (first == nfilms) return;  // no film takes this step: the same for every block
   if (ONE) iters = min(iters, only.P->implicit_iters);
-  CgState* M = ONE ? only.cg : films[0].cg;
-  DevStats* st = ONE ? only.stats : films[0].stats;
+  CgState* M = ONE ? only.cg : films[first].cg;
+  DevStats* st = ONE ? only.stats : films[first].stats;
   uint32_t meet = 0;
   const uint32_t q0 = blockIdx.x * GROUPS + threadIdx.z, dq = gridDim.x * GROUPS;
   const uint32_t nq = (ntiles + SPAN - 1u) / SPAN;

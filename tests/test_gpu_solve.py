@@ -78,3 +78,34 @@ def test_solve_of_many_films_equals_alone(built, films):
         fb.sync()
         ha, hb = fa.read_state()["h"], fb.read_state()["h"]
         assert np.array_equal(ha.view(np.uint32), hb.view(np.uint32))
+
+
+@pytest.mark.parametrize("order", [(0, 1), (0, 0, 1, 0, 1), (1, 0)])
+def test_films_without_implicit_steps_share_a_batch(built, order):
+    """Films with implicit_hydro off (they hold no CG planes), before, among
+    and after films whose frames take implicit steps: each as alone, bit for
+    bit."""
+    from canvaz_film.film import Batch, Film
+    alone, batched = [], []
+    for k, implicit in enumerate(order):
+        cv = pour(40 + 9 * k, 50, k, 2)
+        cv.settings.update(implicit_hydro=implicit)
+        for lst in (alone, batched):
+            f = Film(po.make_settings(cv.settings), cv.w, cv.h, capi.CF_PREC_FP32)
+            f.set_tables(cv.pigtab, cv.cmf)
+            f.write_state(cv.planes)
+            f.update_params(1 / 60, 4)
+            lst.append(f)
+    b = Batch()
+    for f in batched:
+        b.add(f)
+    b.step(2, 4)
+    for f in alone:
+        f.encode_frame(4)
+        f.encode_frame(4)
+    for fa, fb in zip(alone, batched):
+        assert fb.stats()["wet_cells"] > 0
+        fa.sync()
+        ha, hb = fa.read_state()["h"], fb.read_state()["h"]
+        assert np.array_equal(ha.view(np.uint32), hb.view(np.uint32))
+    b.close()
