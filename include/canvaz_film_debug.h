@@ -43,6 +43,13 @@ cf_status cf_debug_run(cf_film* film, const char* kernel, void* stream);
 /* Overwrites the device params with `params` (no re-packing). */
 cf_status cf_debug_set_params(cf_film* film, const cf_params* params);
 
+/* How often a block of the film's implicit solve polls for the others at most
+ * (2^22 by default, some seconds) before it gives the solve up: the film then
+ * keeps its h through that implicit step and cf_get_stats reports
+ * CF_ERR_TIMEOUT.  A batch takes the smallest of its films'; a captured frame
+ * keeps the limit of its capture. */
+cf_status cf_debug_set_wait_limit(cf_film* film, uint32_t polls);
+
 #ifdef __cplusplus
 }
 #endif

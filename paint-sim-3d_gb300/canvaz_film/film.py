@@ -71,6 +71,7 @@ def _lib():
             "cf_debug_write": [vp, C.c_char_p, vp, C.c_size_t],
             "cf_debug_run": [vp, C.c_char_p, vp],
             "cf_debug_set_params": [vp, C.POINTER(Params)],
+            "cf_debug_set_wait_limit": [vp, C.c_uint32],
         }.items():
             fn = getattr(L, name)
             fn.argtypes = args
@@ -271,6 +272,9 @@ class Film:
 
     def set_params(self, p):
         self._check(self.L.cf_debug_set_params(self.p, C.byref(p)), "cf_debug_set_params")
+
+    def set_wait_limit(self, polls):
+        self._check(self.L.cf_debug_set_wait_limit(self.p, polls), "cf_debug_set_wait_limit")
 
     def stats(self):
         s = Stats()

@@ -1040,4 +1040,10 @@ cf_status cf_debug_set_params(cf_film* f, const cf_params* p) {
   return CF_OK;
 }
 
+cf_status cf_debug_set_wait_limit(cf_film* f, uint32_t polls) {
+  if (!f) return CF_ERR_INVALID_ARG;
+  f->meet_polls = polls;
+  return CF_OK;
+}
+
 }  // extern "C"

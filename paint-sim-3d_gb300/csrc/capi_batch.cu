@@ -154,6 +154,7 @@ uint64_t enqueue(cf_batch* b, int p, uint32_t frames, uint32_t substeps, int ada
       V.only = nf == 1u ? &g.films[0]->F : nullptr;
       V.tilted = g.tilted;
       V.few_tiles = g.ntiles <= (uint32_t)b->sms;
+      for (const cf_film* f : g.films) V.meet_polls = std::min(V.meet_polls, f->meet_polls);
       V.persist_blocks = blocks;
       const uint32_t tpb = std::max(b->tune.tiles_per_block, 1u);
       V.tile_grid = tpb > 1u ? (g.ntiles + tpb - 1u) / tpb : 0u;

@@ -346,6 +346,7 @@ __global__ void __launch_bounds__(256) kp_cg_init(CG_ARGS, uint32_t step) {
       S.rz = rz; S.pq = 0.f; S.alpha = 0.f; S.beta = 0.f;
       S.s1x = rz; S.dv = 0.f; S.tv = 0.f; S.s0x = 0.f;
       S.blocks_done = 0u;
+      S.failed = 0u;
     }
   }
 }
@@ -458,9 +459,6 @@ __global__ void __launch_bounds__(256) kp_cg_scalars(const Film* __restrict__ fi
 }
 
 // ---- the iterations without the implicit capillary term, in one launch ----
-// What a block waits at most at a meeting, in polls of a microsecond or so.
-constexpr uint32_t MEET_POLLS = 1u << 22;
-
 __device__ __forceinline__ uint32_t load_relaxed(const uint32_t* p) {
   uint32_t v;
   asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
@@ -485,10 +483,12 @@ __device__ __forceinline__ bool lead_thread() { return threadIdx.x == 0 && threa
 
 // All blocks of a cooperative launch meet: what each wrote before is visible
 // to all after.  `meet` counts the launch's meetings from 1.  Returns false
-// when the wait ran out (counted in the film's stats; the caller leaves).
+// when the wait ran out after `polls`: every film that takes the step then
+// counts it in its stats and keeps its h (kp_cg_finish), and the caller leaves.
 // The wait polls the count of arrivals with relaxed loads and fences once: an
 // acquiring poll empties the SM's L1 each time.
-__device__ __forceinline__ bool blocks_meet(CgState* M, DevStats* st, uint32_t& meet) {
+__device__ __forceinline__ bool blocks_meet(CgState* M, uint32_t& meet, uint32_t polls, const Film* films,
+                                            uint32_t nfilms, uint32_t step) {
   __shared__ uint32_t s_ok;
   ++meet;
   __syncthreads();
@@ -497,8 +497,12 @@ __device__ __forceinline__ bool blocks_meet(CgState* M, DevStats* st, uint32_t& 
     fence_gpu();
     atomicAdd(&M->met, 1u);
     while (load_relaxed(&M->met) < meet * gridDim.x) {
-      if (++k >= MEET_POLLS) {
-        atomicAdd(&st->wait_timeouts, 1u);
+      if (k++ >= polls) {
+        for (uint32_t f = 0; f < nfilms; ++f)
+          if (step < films[f].P->implicit_steps) {
+            atomicAdd(&films[f].stats->wait_timeouts, 1u);
+            films[f].cg->failed = 1u;
+          }
         ok = 0u;
         break;
       }
@@ -628,7 +632,8 @@ constexpr size_t SOLVE_SMEM = sizeof(SolveGroup) * GROUPS;
 // more instructions than the cells).
 template <bool ONE>
 __global__ void __launch_bounds__(256 * GROUPS, PER_SM)
-    kp_cg_solve(const __grid_constant__ Film only, CG_ARGS, uint32_t nfilms, uint32_t step, uint32_t iters) {
+    kp_cg_solve(const __grid_constant__ Film only, CG_ARGS, uint32_t nfilms, uint32_t step, uint32_t iters,
+                uint32_t polls) {
   extern __shared__ __align__(16) unsigned char solve_smem[];
   __shared__ SolveScalars s_one;  // of a film alone
   SolveGroup& G = reinterpret_cast<SolveGroup*>(solve_smem)[threadIdx.z];
@@ -641,7 +646,6 @@ __global__ void __launch_bounds__(256 * GROUPS, PER_SM)
   if (first == nfilms) return;  // no film takes this step: the same for every block
   if (ONE) iters = min(iters, only.P->implicit_iters);
   CgState* M = ONE ? only.cg : films[first].cg;
-  DevStats* st = ONE ? only.stats : films[first].stats;
   uint32_t meet = 0;
   const uint32_t q0 = blockIdx.x * GROUPS + threadIdx.z, dq = gridDim.x * GROUPS;
   const uint32_t nq = (ntiles + SPAN - 1u) / SPAN;
@@ -650,7 +654,7 @@ __global__ void __launch_bounds__(256 * GROUPS, PER_SM)
   // alone for itself (the partials are a few tens of KB in L2), so the blocks
   // meet once a phase; of several films, a group each, and a second meeting.
   auto reduce = [&](uint32_t it, bool after_b) {
-    if (!blocks_meet(M, st, meet)) return false;
+    if (!blocks_meet(M, meet, polls, films, nfilms, step)) return false;
     if (ONE) {
       if (threadIdx.z == 0) {
         const float total = group_total(only, after_b ? only.cg_part2 : only.cg_part, G.sv[0]);
@@ -679,7 +683,7 @@ __global__ void __launch_bounds__(256 * GROUPS, PER_SM)
         F.cg->beta = S.beta;
       }
     }
-    return blocks_meet(M, st, meet);
+    return blocks_meet(M, meet, polls, films, nfilms, step);
   };
   // Walks the spans of the table, the tiles of one film at a time:
   // body(F, span, tx, ty) with the mask of the span's tiles that belong to F
@@ -894,10 +898,11 @@ __global__ void __launch_bounds__(256) kp_cg_lap_u(CG_ARGS, uint32_t step) {
 // film.wgsl:1227-1274 and cg_reduce_mass (film.wgsl:1190-1207).  The new h
 // goes to cg_q (kp_cg_rescale commits it), so every read of a neighbour's h
 // sees the h of before the dispatch.  The final direction of the solve (the
-// reference's last cg_iter_c) is kept in cg_p for later steps' reads.
+// reference's last cg_iter_c) is kept in cg_p for later steps' reads.  A film
+// whose solve was left early keeps its h, acc and cg_p: the step is not taken.
 __global__ void __launch_bounds__(256) kp_cg_finish(CG_ARGS, uint32_t step) {
   CG_TILE
-  if (step >= D.implicit_steps) return;
+  if (step >= D.implicit_steps || F.cg->failed != 0u) return;
   __shared__ float sv[256];
   __shared__ __align__(16) float stv[256];
   __shared__ uint32_t s_moved;
@@ -972,8 +977,9 @@ __global__ void __launch_bounds__(256) kp_cg_finish(CG_ARGS, uint32_t step) {
 __global__ void __launch_bounds__(256) kp_cg_rescale(CG_ARGS, uint32_t step) {
   CG_TILE
   if (step >= D.implicit_steps || !cell_on) return;
-  const float hn = F.cg_q[c];
   const CgState& S = *F.cg;
+  if (S.failed != 0u) return;
+  const float hn = F.cg_q[c];
   if (S.tv <= 0.f) {
     F.hh[c] = hn;
     return;
@@ -1007,9 +1013,9 @@ uint32_t launch_cg_step(const PackedFrame& V, int mode, uint32_t step, uint32_t 
     }
   } else {
     kp_cg_init<true><<<nt, b, 0, st>>>(A, T, nt, step);
-    uint32_t nfilms = V.nfilms, ntiles = nt;
+    uint32_t nfilms = V.nfilms, ntiles = nt, polls = V.meet_polls;
     Film only = V.only != nullptr ? *V.only : Film{};
-    void* args[] = {&only, &A, &T, &ntiles, &nfilms, &step, &iters};
+    void* args[] = {&only, &A, &T, &ntiles, &nfilms, &step, &iters, &polls};
     // an error stays with the runtime for the caller's check of the launches
     cudaLaunchCooperativeKernel(V.only != nullptr ? (const void*)kp_cg_solve<true> : (const void*)kp_cg_solve<false>,
                                 dim3(solve_blocks(nt)), dim3(16, 16, GROUPS), args, SOLVE_SMEM, st);

@@ -54,10 +54,11 @@ struct alignas(128) CgState {
   float rz, pq, alpha, beta;  // cg_s[0]
   float s1x, dv, tv, s0x;     // cg_s[1]: rz of the init, sum of h changes, sum of h, last rz
   uint32_t blocks_done;
+  uint32_t failed;  // the step's solve was left before its last iteration: the step keeps h
   // the meeting point of the solve's blocks (the first film's that takes the step), on a
   // line of its own that the waiting blocks poll: how many arrivals, and how
   // many blocks have left; zero between launches
-  uint32_t pad[23];
+  uint32_t pad[22];
   uint32_t met, left;
   uint32_t pad2[30];
 };

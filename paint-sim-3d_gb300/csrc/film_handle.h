@@ -34,6 +34,7 @@ struct cf_film {
   uint32_t frames = 0;
   uint64_t launches = 0;  // kernels enqueued by this film
   int device = 0, sms = 0;
+  uint32_t meet_polls = cfk::MEET_POLLS;  // cfk::PackedFrame::meet_polls of the film
   std::string err;
   cf_batch* batch = nullptr;  // the batch this film steps in, if any
   // the film's own packed view: its record as created and with the strata
@@ -63,6 +64,7 @@ inline cfk::PackedFrame solo_view(const cf_film* f) {
   V.tiles = nullptr;  // the identity table over this film
   V.only = &f->F;
   V.tilted = film_tilted(f);
+  V.meet_polls = f->meet_polls;
   V.ntiles = f->tw * f->th;
   V.few_tiles = V.ntiles <= (uint32_t)std::max(f->sms, 1);
   V.nfilms = 1;

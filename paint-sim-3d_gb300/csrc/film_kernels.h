@@ -12,6 +12,7 @@ namespace cfk {
 // stepped alone is a view of its own two records and tiles; a batch is a view
 // of many films; both run the same compiled kernels, so a film's result does
 // not depend on what else shares the launch.
+constexpr uint32_t MEET_POLLS = 1u << 22;
 struct PackedFrame {
   const Film* films;       // device array: the films as the frame starts
   const Film* films_next;  // the same films with the strata generations swapped
@@ -27,6 +28,9 @@ struct PackedFrame {
   // path run: whether any film is tilted, and whether there is at most one tile
   // per SM in all.  Every instance gives a film the same bits.
   bool tilted = true, few_tiles = false;
+  // what a block of the implicit solve waits at most at a meeting, in polls of
+  // a microsecond or so
+  uint32_t meet_polls = MEET_POLLS;
   // implicit hydrostatic steps launched (each film's kernels skip the steps
   // beyond its own count), CG iterations per step (each film stops at its
   // own), and whether any film has the implicit capillary term

@@ -109,3 +109,59 @@ def test_films_without_implicit_steps_share_a_batch(built, order):
         ha, hb = fa.read_state()["h"], fb.read_state()["h"]
         assert np.array_equal(ha.view(np.uint32), hb.view(np.uint32))
     b.close()
+
+
+@pytest.mark.parametrize("films", [1, 3])
+def test_a_solve_that_gives_up_is_reported_by_every_film(built, films):
+    """With a limit of no polls the first block to wait at a meeting leaves the
+    solve and the others follow: the kernel returns, every film of the launch
+    reports the timeout and keeps its h through the implicit step, and the next
+    frame, with the default limit, solves as a film that never gave up."""
+    from canvaz_film.film import Batch, Film
+    fs, ref, keep = [], [], []
+    for k in range(films):
+        cv = pour(150 + 16 * k, 130, k, 4)  # 90 tiles and more: 12 or more blocks
+        cv.settings.update(all_active=1)
+        for lst in (fs, ref, keep):
+            st = po.make_settings(dict(cv.settings, implicit_hydro=int(lst is not keep)))
+            f = Film(st, cv.w, cv.h, capi.CF_PREC_FP32)
+            f.set_tables(cv.pigtab, cv.cmf)
+            f.write_state(cv.planes)
+            f.update_params(1 / 60, 1)
+            lst.append(f)
+
+    def step(lst):
+        b = Batch()  # a batch captures its frames with the limit of the time
+        for f in lst:
+            b.add(f)
+        b.step(1, 1)
+        for f in lst:
+            f.sync()
+        b.close()
+
+    for f in fs:
+        f.set_wait_limit(0)
+    step(fs)
+    for f in fs:
+        with pytest.raises(capi.FilmError) as e:
+            f.stats()
+        assert e.value.status == capi.CF_ERR_TIMEOUT
+    step(keep)  # the same frame of films that take no implicit steps
+    step(ref)
+    for f, g, r in zip(fs, keep, ref):
+        h = f.read_state()["h"]
+        assert np.array_equal(h, g.read_state()["h"])
+        assert not np.array_equal(h, r.read_state()["h"])
+    # later frames: those of a film that is written the same state
+    for f, g in zip(fs, ref):
+        g.write_state(f.read_state())
+        s = f.read_state()
+        f.write_state(s)
+        for x in (f, g):
+            x.set_wait_limit(1 << 22)
+            x.update_params(1 / 60, 1)
+    step(fs)
+    step(ref)
+    for f, g in zip(fs, ref):
+        assert g.stats()["wet_cells"] > 0
+        assert np.array_equal(f.read_state()["h"], g.read_state()["h"])
