@@ -27,6 +27,8 @@
 // kernels.  A neighbour in an inactive tile
 // is read as the reference reads it: its cg_m and cg_p as the last step that
 // covered it left them.
+#include <cuda.h>
+
 #include <algorithm>
 #include <mutex>
 
@@ -868,11 +870,41 @@ __global__ void __launch_bounds__(256 * GROUPS, PER_SM)
   blocks_leave(M);
 }
 
-// The grid of kp_cg_solve: every block that fits the device at once, no more
-// than the tiles fill.
-uint32_t solve_blocks(uint32_t ntiles) {
+// The SMs that work enqueued on `st` may run on: those of the stream's green
+// context where it has one, else all of the device's `sms`.
+uint32_t stream_sms(cudaStream_t st, uint32_t sms) {
+  using GetCtx = CUresult (*)(CUstream, CUcontext*, CUgreenCtx*);
+  using GetRes = CUresult (*)(CUgreenCtx, CUdevResource*, CUdevResourceType);
+  static GetCtx get_ctx = nullptr;
+  static GetRes get_res = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {  // through the runtime: the library does not link the driver library
+    cudaDriverEntryPointQueryResult q{};
+    void *c = nullptr, *r = nullptr;
+    if (cudaGetDriverEntryPointByVersion("cuStreamGetCtx", &c, 12050, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess &&
+        cudaGetDriverEntryPointByVersion("cuGreenCtxGetDevResource", &r, 12040, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess) {
+      get_ctx = reinterpret_cast<GetCtx>(c);
+      get_res = reinterpret_cast<GetRes>(r);
+    }
+    cudaGetLastError();
+  });
+  CUcontext ctx = nullptr;
+  CUgreenCtx green = nullptr;
+  CUdevResource res;
+  if (get_ctx == nullptr || get_ctx(st, &ctx, &green) != CUDA_SUCCESS || green == nullptr ||
+      get_res(green, &res, CU_DEV_RESOURCE_TYPE_SM) != CUDA_SUCCESS)
+    return sms;
+  return std::min<uint32_t>(sms, std::max(res.sm.smCount, 1u));
+}
+
+// The grid of kp_cg_solve: every block that fits at once on the SMs the stream
+// has (a larger cooperative launch is refused), no more than the tiles fill.
+// The sums do not depend on it.
+uint32_t solve_blocks(uint32_t ntiles, cudaStream_t st) {
   static std::mutex mu;
-  static int per_device[64] = {};
+  static int per_device[64] = {}, sms_of[64] = {};  // blocks an SM, SMs
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1u;
   std::lock_guard<std::mutex> lock(mu);
@@ -883,9 +915,11 @@ uint32_t solve_blocks(uint32_t ntiles) {
     cudaFuncSetAttribute(kp_cg_solve<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SOLVE_SMEM);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&a, kp_cg_solve<true>, 256 * GROUPS, SOLVE_SMEM);
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, kp_cg_solve<false>, 256 * GROUPS, SOLVE_SMEM);
-    per_device[dev] = std::max(sms * std::min(a, b), 1);
+    per_device[dev] = std::max(std::min(a, b), 1);
+    sms_of[dev] = std::max(sms, 1);
   }
-  return std::min<uint32_t>((uint32_t)per_device[dev], (ntiles + GROUPS * SPAN - 1u) / (GROUPS * SPAN));
+  return std::min<uint32_t>((uint32_t)per_device[dev] * stream_sms(st, (uint32_t)sms_of[dev]),
+                            (ntiles + GROUPS * SPAN - 1u) / (GROUPS * SPAN));
 }
 
 // cg_lap_u (film.wgsl:1080-1085), only with the implicit capillary term
@@ -1018,7 +1052,7 @@ uint32_t launch_cg_step(const PackedFrame& V, int mode, uint32_t step, uint32_t 
     void* args[] = {&only, &A, &T, &ntiles, &nfilms, &step, &iters, &polls};
     // an error stays with the runtime for the caller's check of the launches
     cudaLaunchCooperativeKernel(V.only != nullptr ? (const void*)kp_cg_solve<true> : (const void*)kp_cg_solve<false>,
-                                dim3(solve_blocks(nt)), dim3(16, 16, GROUPS), args, SOLVE_SMEM, st);
+                                dim3(solve_blocks(nt, st)), dim3(16, 16, GROUPS), args, SOLVE_SMEM, st);
     n += 1;
   }
   if (cap_implicit) { kp_cg_lap_u<<<nt, b, 0, st>>>(A, T, nt, step); ++n; }
