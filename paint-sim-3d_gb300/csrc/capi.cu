@@ -132,6 +132,16 @@ cf_status upload_params(cf_film* f, cudaStream_t st, float dt_max) {
   return CF_OK;
 }
 
+// The view of a frame enqueued on `st`.  Under capture the instances that serve
+// tilted films too: the graph may be replayed after a clone of one.
+static cfk::PackedFrame frame_view(const cf_film* f, cudaStream_t st) {
+  cfk::PackedFrame V = solo_view(f);
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cs) != cudaSuccess) cudaGetLastError();
+  V.tilted = V.tilted || cs != cudaStreamCaptureStatusNone;
+  return V;
+}
+
 static cf_status check_launch(cf_film* f) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) {
@@ -772,7 +782,7 @@ cf_status cf_encode_frame(cf_film* f, uint32_t substeps, void* stream) {
   cf_status s = upload_params(f, st);
   if (s != CF_OK) return s;
   f->launches += launch_pending_deposits(f, st);
-  cfk::PackedFrame V = solo_view(f);
+  cfk::PackedFrame V = frame_view(f, st);
   V.implicit_steps = f->S.implicit_hydro ? f->implicit_steps : 0u;
   f->launches += cfk::launch_frame_packed(V, f->prec, substeps, 0, st);
   swap_generations(f);
@@ -789,7 +799,7 @@ cf_status cf_step_adaptive(cf_film* f, float dt_max, void* stream) {
   cf_status s = upload_params(f, st, dt_max);
   if (s != CF_OK) return s;
   f->launches += launch_pending_deposits(f, st);
-  cfk::PackedFrame V = solo_view(f);
+  cfk::PackedFrame V = frame_view(f, st);
   // the device picks dt and with it the implicit step count (0..4): the
   // launches cover 4 steps and the film's kernels skip the ones it does not take
   V.implicit_steps = f->S.implicit_hydro ? 4u : 0u;
