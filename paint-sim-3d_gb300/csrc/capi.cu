@@ -1031,12 +1031,15 @@ cf_status cf_debug_run(cf_film* f, const char* kernel, void* stream) {
   cudaStream_t st = (cudaStream_t)stream;
   cf_status s = upload_params(f, st);
   if (s != CF_OK) return s;
-  CUDA_TRY(f, cudaMemsetAsync(f->F.tile_still, 0, 4 * (size_t)f->tw * f->th, st));  // every tile takes part
+  // every tile takes part, and no frame was around the dispatch for a level it raises
+  const size_t still_bytes = 4 * (size_t)f->tw * f->th;
+  CUDA_TRY(f, cudaMemsetAsync(f->F.tile_still, 0, still_bytes, st));
   const int r = std::strcmp(kernel, "deposit") == 0 ? (launch_pending_deposits(f, st), 1)
                                                     : cfk::launch_one(solo_view(f), f->prec, kernel, st);
   if (!r) return fail(f, CF_ERR_INVALID_ARG, "unknown kernel");
   if (r == 2) swap_generations(f);
   if ((s = check_launch(f)) != CF_OK) return s;
+  CUDA_TRY(f, cudaMemsetAsync(f->F.tile_still, 0, still_bytes, st));
   CUDA_TRY(f, cudaStreamSynchronize(st));
   return CF_OK;
 }
