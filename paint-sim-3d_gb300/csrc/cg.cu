@@ -12,8 +12,10 @@
 //    the active tiles that hold paint: phase a forms the search direction
 //    p_k = r / d + beta p_{k-1} of the tile and its halo on the fly (so the
 //    reference's cg_iter_c needs no pass of its own) and computes q = A p_k,
-//    phase b updates r; between the phases the blocks meet, and the last to
-//    arrive sums the tiles' partials and updates the film's scalars.  With the
+//    phase b updates r; after each phase the blocks meet, and the tiles'
+//    partials are summed and the film's scalars updated: of a film alone by
+//    every block for itself, of several by one group of threads a film, after
+//    which the blocks meet again.  With the
 //    implicit capillary term (off by default) the iterations are separate
 //    launches instead (kp_cg_lap_p, kp_cg_iter_a, kp_cg_iter_b and
 //    kp_cg_scalars), which also form the Laplacian of the direction;
@@ -21,12 +23,10 @@
 //    (neighbours read h as of before the dispatch), the final direction into
 //    cg_p; kp_cg_rescale: the mass correction and the h commit.
 // Each sum over a film (p.q, r.z, the mass change) is a per-tile tree sum
-// and the film's total of them in tile order: by the last block to arrive in
-// the solve, by the last block to finish (an atomic count, no waiting) in the
-// once-per-step
-// kernels.  A neighbour in an inactive tile
-// is read as the reference reads it: its cg_m and cg_p as the last step that
-// covered it left them.
+// and the film's total of them in tile order; in the once-per-step kernels it
+// is formed by the last block to finish (an atomic count, no waiting).  A
+// neighbour in an inactive tile is read as the reference reads it: its cg_m and
+// cg_p as the last step that covered it left them.
 #include <cuda.h>
 
 #include <algorithm>

@@ -174,9 +174,9 @@ struct Film {
 // resets the state to SHADE_NONE.  SHADE_DRY: the colour holds the dry cell's colour,
 // which depends only on the substrate, the relief and the CMF table.
 // SHADE_DRY2: the same, and the strata pass has written zero thicknesses and
-// cure fractions for the cell into both strata generations (it was dry in an
-// active tile two passes running), so a pass that finds it dry again has
-// nothing to read or write for it.
+// cure fractions for the cell into both strata generations (it was dry two
+// passes running), so a pass that finds it dry again has nothing to read or
+// write for it.
 constexpr uint8_t SHADE_NONE = 0, SHADE_DRY = 1, SHADE_WET = 2, SHADE_DRY2 = 3;
 // Film::tile_still of a 16x16 tile.  A frame writes the same values into
 // every plane of a tile without paint again and again: no height, rate, flux,
@@ -192,8 +192,8 @@ constexpr uint8_t SHADE_NONE = 0, SHADE_DRY = 1, SHADE_WET = 2, SHADE_DRY2 = 3;
 // one cell nearer with each substep, so a tile 16 cells or more from any is out
 // of reach of a frame of at most STILL_SUBSTEPS of them (a cell reads at most
 // 4 cells around it).  Whatever else writes a film's planes (state uploads,
-// tables, inspection, dry_now) clears the levels; deposits set the tile's
-// moved word.
+// tables, inspection, dry_now) clears the levels, inspection after its
+// dispatch too; deposits set the tile's moved word.
 constexpr uint32_t STILL_SLEEP = 1u, STILL_AWAKE = 2u, STILL_LEVEL = 3u, STILL_DRY9 = 64u, STILL_QUIET = 128u;
 constexpr uint32_t STILL_SUBSTEPS = 8u;
 // Planes staged by tensor loads (the flow, laplacian, limiter + apply and

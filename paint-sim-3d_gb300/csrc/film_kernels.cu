@@ -592,24 +592,21 @@ struct TileFaces {
   uint8_t cell[4][256];
   uint32_t count[4];
 };
-// Lists face k of the cell in slot `slot` of the tile (y * 16 + x) when
-// `live` (every thread of the block calls this, with the same k).
-__device__ __forceinline__ void tile_faces_add(TileFaces& S, int k, bool live, int slot) {
-  const int lane = (int)(threadIdx.y * 16 + threadIdx.x) & 31;
+// Lists face k of the thread's cell when `live` (every thread of the block
+// calls this, with the same k).
+__device__ __forceinline__ void tile_faces_add(TileFaces& S, int k, bool live) {
+  const int slot = (int)(threadIdx.y * 16 + threadIdx.x), lane = slot & 31;
   const unsigned m = __ballot_sync(0xffffffffu, live);
   uint32_t base = 0;
   if (lane == 0 && m) base = atomicAdd(&S.count[k], (uint32_t)__popc(m));
   base = __shfl_sync(0xffffffffu, base, 0);
   if (live) S.cell[k][base + __popc(m & ((1u << lane) - 1u))] = (uint8_t)slot;
 }
-__device__ __forceinline__ void tile_faces_add(TileFaces& S, int k, bool live) {
-  tile_faces_add(S, k, live, (int)(threadIdx.y * 16 + threadIdx.x));
-}
-// Runs fn(k, i, j, c) for every listed face, the block's NT threads in turn.
-template <int NT = 256, class Fn>
+// Runs fn(k, i, j, c) for every listed face, the block's 256 threads in turn.
+template <class Fn>
 __device__ __forceinline__ void tile_faces_each(const Film& F, TileId T, const TileFaces& S, Fn fn) {
   const uint32_t n0 = S.count[0], n1 = n0 + S.count[1], n2 = n1 + S.count[2], n3 = n2 + S.count[3];
-  for (uint32_t e = threadIdx.y * 16 + threadIdx.x; e < n3; e += NT) {
+  for (uint32_t e = threadIdx.y * 16 + threadIdx.x; e < n3; e += 256u) {
     const int k = e < n0 ? 0 : e < n1 ? 1 : e < n2 ? 2 : 3;
     const uint32_t base = k == 0 ? 0u : k == 1 ? n0 : k == 2 ? n1 : n2;
     const uint32_t t = S.cell[k][e - base];
@@ -655,9 +652,9 @@ __device__ __forceinline__ void fluxes_tile(const Film& F, TileId T) {
 // the tile + 1 ring (what the faces read), then the faces.  Each value is the
 // expression the separate kernels evaluate, so the fluxes are the separate
 // dispatches' to rounding.  The plug mobilities of the tile go to the tmp
-// plane (strata_split reads the last substep's); the pressures stay on chip:
-// laplacian is dispatched again before strata_split, and no other kernel
-// reads them in between.
+// plane (a neighbour that wakes later reads a sleeping tile's there); the
+// pressures stay on chip: the split evaluates its own from the last heights,
+// and no other kernel reads them in between.
 constexpr uint32_t FLOW_WAIT_POLLS = 1u << 22;
 // What the tiles that evaluate faces hold (PtTile reads it).
 struct FaceSmem {
@@ -1394,48 +1391,34 @@ __device__ __forceinline__ void flow_tile(const Film& F, TileId T) {
 // zeroing.
 template <int MODE, int NT>
 __device__ __forceinline__ void strata_split_tile(const Film& F, TileId T) {
-  constexpr int R = NT < 256 ? 256 / NT : 1;  // own cells a thread (slots tid, tid + NT, ...)
   __shared__ __align__(128) SplitSmem S;
   if (!tile_runs(F, T)) return;
   const DevParams& D = *F.P;
   const cf_params& P = D.p;
   const int tid = threadIdx.y * 16 + threadIdx.x;
   const int i0 = (int)T.x * 16, j0 = (int)T.y * 16;
-  const int i = i0 + (tid & 15);
-  bool in[R];
-  uint32_t c[R];
-  float4 a4[R];
-#pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int j = j0 + ((tid + NT * r) >> 4);
-    in[r] = tid < 256 && i < (int)F.w && j < (int)F.h;
-    c[r] = in[r] ? idx(F, i, j) : 0u;
-    a4[r] = in[r] ? F.acc[c[r]] : make_float4(0.f, 0.f, 0.f, 0.f);
-    if (tid < 256) S.flags[tid + NT * r] = 0u;
-  }
+  // the tile's own cell of the first 256 threads
+  const int i = i0 + (tid & 15), j = j0 + (tid >> 4);
+  const bool in = tid < 256 && i < (int)F.w && j < (int)F.h;
+  const uint32_t c = in ? idx(F, i, j) : 0u;
+  const float4 a4 = in ? F.acc[c] : make_float4(0.f, 0.f, 0.f, 0.f);
+  if (tid < 256) S.flags[tid] = 0u;
   tile_acts(F, S, T, tid);
   if (tid == 0) S.nface = 0u;
   if (!stage_box<MODE, false, SplitSmem, NT>(F, S, i0, j0, tid)) return;
   tile_surface<SplitSmem, NT>(F, P, S, i0, j0, tid);
   if (tid < 256) {
+    bool want[4];
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int j = j0 + ((tid + NT * r) >> 4);
-      bool want[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) want[k] = in[r] && sel4(a4[r], k) != 0.f && in_grid(F, i + FACE_DI[k], j + FACE_DJ[k]);
-      smem_append4(S.face, &S.nface, want, tid + NT * r);
-    }
+    for (int k = 0; k < 4; ++k) want[k] = in && sel4(a4, k) != 0.f && in_grid(F, i + FACE_DI[k], j + FACE_DJ[k]);
+    smem_append4(S.face, &S.nface, want, tid);
   }
   __syncthreads();
   const uint32_t nf = S.nface;
   if (nf == 0u) {
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const int ty = (tid + NT * r) >> 4;
-      if (!in[r]) continue;
-      F.pres[c[r]] = tile_pres(F, P, S, i0, j0, (tid & 15) + 1, ty + 1, i, j0 + ty, c[r]);
-      F.fflags[c[r]] = 0u;
+    if (in) {
+      F.pres[c] = tile_pres(F, P, S, i0, j0, (tid & 15) + 1, (tid >> 4) + 1, i, j, c);
+      F.fflags[c] = 0u;
     }
     return;
   }
@@ -1472,9 +1455,7 @@ __device__ __forceinline__ void strata_split_tile(const Film& F, TileId T) {
     if (o.x != 0.f || o.y != 0.f || o.z != 0.f || o.w != 0.f) atomicOr(&S.flags[f & 255u], 1u << k);
   }
   __syncthreads();
-#pragma unroll
-  for (int r = 0; r < R; ++r)
-    if (in[r]) F.fflags[c[r]] = S.flags[tid + NT * r];
+  if (in) F.fflags[c] = S.flags[tid];
 }
 
 __device__ __forceinline__ void load_tables(const Film& F, float* tab, float* cm, float* ltab, int tid, int nthreads) {
@@ -2377,10 +2358,11 @@ __global__ void __launch_bounds__(256, 6) kp_fluxes(PACKED_ARGS) { PACKED_TILES(
 // long enough that a walk has nothing to hide), and one instance for the
 // precision modes of one rheology type.  Bound by instruction issue on canvases
 // of many wet tiles, by the chain of a tile's phases on small ones.  256 threads
-// a tile where there are many tiles: flow at 5 blocks an SM (48 registers; at 6
-// or more the faces spill: 1200 x 800 pours 75 us a substep against 80, 2048^2
-// drips 216 against 221, 4096^2 blobs 529 against 518), split at 8 (2048^2 pours
-// 402 us, 4096^2 blobs 205 against 379 and 232 at 6).  No more tiles in all than
+// a tile where there are many tiles: flow at 5 blocks an SM (48 registers, some 50
+// bytes a thread spilled; against 6 blocks of 40 registers 1200 x 800 pours 75 us
+// a substep and 80, 2048^2 drips 216 and 221, 4096^2 blobs 529 and 518), split at
+// 8 (32 registers, 156 bytes spilled, but the tiles in flight count for more:
+// 2048^2 pours 402 us, 4096^2 blobs 205, against 379 and 232 at 6).  No more tiles in all than
 // SMs (FEW) wait for the longest chain of a tile instead: 512 threads halve its
 // rounds of faces (64^2: 131 us a frame against 144).  The instances give the
 // same bits, so a batch takes one for all of its films: kept apart by size, 9

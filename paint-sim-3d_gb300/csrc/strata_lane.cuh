@@ -264,8 +264,8 @@ __device__ __forceinline__ void lane_add_band(const Lanes<N>& H, LaneStack<N>& s
   if (above > 1e-14f) lane_push_top(H, s, above, pin, cv, tiny, close_d);
 }
 
-// CellAcc with one band per lane: the composition sums are half-warp sums
-// over the 12 pigment lanes, the reflectance of band q stays in lane q.
+// CellAcc with N bands per lane: the composition sums are sums over the cell's
+// lanes of the 12 pigment slots, the reflectance of a band stays in its lane.
 template <int N>
 struct LaneAcc {
   float total, lnmu, tau, thin, wsum, nsum, nw;  // equal on all lanes
@@ -282,7 +282,7 @@ struct LaneAcc {
 #pragma unroll
     for (int u = 0; u < N; ++u) r[u] = h16_to_f(rf[H.slot(u)]);
   }
-  // xs: 32 floats of the half-warp's shared memory, 16-byte aligned, where
+  // xs: 32 floats of the cell's shared memory, 16-byte aligned, where
   // the lanes leave their slot and pigment weight for the others to read
   // (four vector loads instead of sixteen shuffles)
   __device__ __forceinline__ void add(const Lanes<N>& H, int k, float t, float cure, const float (&pg)[N], float hv,
