@@ -133,6 +133,20 @@ def step_traffic(workload):
     return None
 
 
+def step_roofline(cell_steps, seconds, alg, traffic_pc, peak, peak_kind, scope):
+    """The roofline entry of a film step: its DRAM traffic over the measured
+    bandwidth where the traffic is known, else the algorithmic bytes, which
+    count every persistent plane of every cell.  A step leaves out most of
+    those on canvases that are mostly dry, so their rate stands beside the
+    fraction and is not one (it can pass the peak)."""
+    gbs = lambda per_cell: per_cell * cell_steps / seconds / 1e9  # noqa: E731
+    known = traffic_pc is not None
+    achieved = gbs(traffic_pc if known else alg)
+    return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+            "peak_source": peak_kind, "basis": "measured DRAM traffic" if known else "algorithmic bytes",
+            "alg_bytes_per_cell": alg, "alg_gbs": gbs(alg), "scope": scope}
+
+
 class _Nvml:
     """Read-only NVML queries through ctypes (the driver's libnvidia-ml):
     SM clock, its maximum, power and the active clock-event reasons."""
@@ -895,7 +909,6 @@ def gpu_arm(args):
     value = world * cells * args.steps / t / 1e9
     alg = ALG_BYTES_PER_CELL[prec]
     peak, peak_kind = peaks()
-    achieved = alg * cells * args.steps / t / 1e9
     traffic_pc = step_traffic(args.workload)
     mass0 = s0["wet_volume"] + s0["relief_volume"]
     mass1 = s1["wet_volume"] + s1["relief_volume"]
@@ -1006,12 +1019,10 @@ def gpu_arm(args):
             torch.distributed.all_reduce(tt, op=torch.distributed.ReduceOp.MAX)
             tb = float(tt.item())
         pb = WORKLOADS[twin][1]
-        ab = ALG_BYTES_PER_CELL[pb] * cells * args.steps / tb / 1e9
         bf16 = {"workload": twin, "value": world * cells * args.steps / tb / 1e9, "unit": "Gcell-updates/s",
                 "ms_per_step": 1e3 * tb / args.steps, "dtype": PREC_NAME[pb], "gpu_launches": int(lb),
-                "roofline": {"bound": "hbm", "achieved": ab, "peak": peak, "unit": "GB/s", "frac": ab / peak,
-                             "peak_source": peak_kind, "alg_bytes_per_cell": ALG_BYTES_PER_CELL[pb],
-                             "scope": "whole step (all kernels of cf_encode_frame)"}}
+                "roofline": step_roofline(cells * args.steps, tb, ALG_BYTES_PER_CELL[pb], step_traffic(twin), peak,
+                                          peak_kind, "whole step (all kernels of cf_encode_frame)")}
         fb.close()
     cb = None
     if rank == 0 and not args.no_cpu_baseline:
@@ -1024,12 +1035,10 @@ def gpu_arm(args):
             "higher_is_better": True, "scaling": "weak", "vs_baseline": None, "dtype": PREC_NAME[prec],
             "data": "synthetic (seeded drip polylines / Gaussian blobs; no public dataset)",
             "config": single_config(args.workload, cv, prec, adaptive, dt_max, world),
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
-                         "frac": achieved / peak, "peak_source": peak_kind,
-                         "alg_bytes_per_cell": alg,
-                         "scope": "whole step (all kernels of %s)" % ("cf_step_adaptive" if adaptive
-                                                                      else "cf_encode_frame"),
-                         "traffic": None if traffic_pc is None else traffic_pc * cells},
+            "roofline": dict(step_roofline(cells * args.steps, t, alg, traffic_pc, peak, peak_kind,
+                                           "whole step (all kernels of %s)" % ("cf_step_adaptive" if adaptive
+                                                                               else "cf_encode_frame")),
+                             traffic=None if traffic_pc is None else traffic_pc * cells),
             "gpu_launches": int(launches),
             "clocks": clocks,
             "e2e": e2e,
