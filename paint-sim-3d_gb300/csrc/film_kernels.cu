@@ -2356,8 +2356,10 @@ template <int MODE, bool WALK = false>
 __global__ void __launch_bounds__(256, 6) kp_fluxes(PACKED_ARGS) { PACKED_TILES(WALK, fluxes_tile<MODE>(F, T)) }
 // The kernels that evaluate faces: one tile a block always (their tiles are
 // long enough that a walk has nothing to hide), and one instance for the
-// precision modes of one rheology type.  Bound by instruction issue on canvases
-// of many wet tiles, by the chain of a tile's phases on small ones.  256 threads
+// precision modes of one rheology type.  Bound by instruction issue and by the
+// loads and barriers between a tile's phases (1024^2 blobs, flow: an instruction
+// in 59 % of the cycles, a warp's next one after 14, 4 of them for a load and 2
+// at a barrier), by the chain of the phases alone on small canvases.  256 threads
 // a tile where there are many tiles: flow at 5 blocks an SM (48 registers, some 50
 // bytes a thread spilled; against 6 blocks of 40 registers 1200 x 800 pours 75 us
 // a substep and 80, 2048^2 drips 216 and 221, 4096^2 blobs 529 and 518), split at
@@ -2443,8 +2445,9 @@ __global__ void kp_stats_reset(const Film* __restrict__ films, uint32_t nfilms) 
   if (f < nfilms) stats_reset_film(films[f]);
 }
 // The strata full path over every film's list, with the film's tables.  Bound
-// by issue: most instructions are what all lanes of a cell compute alike, so
-// many tiles take a quarter-warp to a cell (the listed cells of 2048^2 drips
+// by the instructions a cell takes, in issue (an instruction in 51 % of the cycles
+// at 1024^2 drips), their loads and their fetch: most are what all lanes of a
+// cell compute alike, so many tiles take a quarter-warp to a cell (the listed cells of 2048^2 drips
 // 315 -> 257 us, 2048^2 pours after a step of heavy flow 2777 -> 1746, 1200x800
 // at 64 substeps 630 -> 381).  At most one tile per SM in all (FEW) keeps the
 // half-warp: the lists are one round of the chip, and a cell's latency is what

@@ -14,7 +14,9 @@
 // and the tile activity flags.  The camera is the renderer's uniform as the
 // caller fills it (cf_render_cam, the layout of render.wgsl:1-15).
 //
-// Bound by instruction fetch, then issue: the march, the bisection, the ambient
+// Bound by instructions, once by their fetch, now by issue (an instruction in 64 %
+// of the cycles of a 960x540 view; of a warp's 11 cycles an instruction 3 wait at
+// a meeting point, 0.7 for a fetch): the march, the bisection, the ambient
 // occlusion and the slopes evaluate the weave some 37 times a pixel of bare
 // canvas, about a thousand instructions each.  So the plain renderer is compiled
 // without the beauty mode's code, the warps of a block keep in step through the
@@ -22,7 +24,7 @@
 // decide the comparison it feeds (BUMP_LO, BUMP_HI): 1920x1080 over bare and
 // painted canvas 2620 -> 1450 us (2476 with the split alone, 2234 with the
 // bounds, then in step 1752 at 32 x 32 threads a block, 1550 at 16 x 32, 1450
-// with five more meeting points after the bisection; 1496 now that finished
+// with five more meeting points after the bisection; 1475 now that finished
 // pixels and lanes outside the picture pass the meeting points too).
 //
 // Every function follows the shader's f32 arithmetic in its order of
@@ -1171,8 +1173,8 @@ __device__ __forceinline__ void fs(const R& X, bool live, float2 ndc_in, const T
 // of instructions among 16 warps, but its warps wait for the slowest of 512
 // pixels and it fills the chip in coarser steps, so it is for views of at least
 // three rounds of the chip; below, four warps.  16 x 32 against 16 x 8 (us):
-// 1600x900 830 and 987, 960x540 464 and 503, 800x450 411 and 370, 640x360 387
-// and 294, 218x123 310 and 227 (16 x 8 out of step 1105, 562, 401, 323, 226).
+// 1600x900 843 and 1014, 1216x673 428 and 468, 960x540 470 and 518, 800x450 416
+// and 378, 640x360 394 and 299, 452x258 267 and 208, 218x123 314 and 229.
 constexpr uint32_t LIT_W = 16, LIT_ROWS = 32, LIT_ROWS_SMALL = 8, LIT_ROUNDS = 3;
 // One thread per pixel of a width x height target; the pixel centre's ndc as
 // the full-screen triangle interpolates it (y up).
