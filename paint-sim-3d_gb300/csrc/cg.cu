@@ -483,23 +483,12 @@ __device__ __forceinline__ void group_sync() {
 }
 __device__ __forceinline__ bool lead_thread() { return threadIdx.x == 0 && threadIdx.y == 0 && threadIdx.z == 0; }
 
-// Marks every film that takes the step as left early (out of line: the path
-// that no launch takes keeps no registers of the solve's).
-__device__ __noinline__ void give_up(const Film* films, uint32_t nfilms, uint32_t step) {
-  for (uint32_t f = 0; f < nfilms; ++f)
-    if (step < films[f].P->implicit_steps) {
-      atomicAdd(&films[f].stats->wait_timeouts, 1u);
-      films[f].cg->failed = 1u;
-    }
-}
 // All blocks of a cooperative launch meet: what each wrote before is visible
 // to all after.  `meet` counts the launch's meetings from 1.  Returns false
-// when the wait ran out after `polls`: every film that takes the step then
-// counts it in its stats and keeps its h (kp_cg_finish), and the caller leaves.
+// when the wait ran out after `polls`: the caller leaves the solve.
 // The wait polls the count of arrivals with relaxed loads and fences once: an
 // acquiring poll empties the SM's L1 each time.
-__device__ __forceinline__ bool blocks_meet(CgState* M, uint32_t& meet, uint32_t polls, const Film* films,
-                                            uint32_t nfilms, uint32_t step) {
+__device__ __forceinline__ bool blocks_meet(CgState* M, uint32_t& meet, uint32_t polls) {
   __shared__ uint32_t s_ok;
   ++meet;
   __syncthreads();
@@ -509,7 +498,6 @@ __device__ __forceinline__ bool blocks_meet(CgState* M, uint32_t& meet, uint32_t
     atomicAdd(&M->met, 1u);
     while (load_relaxed(&M->met) < meet * gridDim.x) {
       if (k++ >= polls) {
-        give_up(films, nfilms, step);
         ok = 0u;
         break;
       }
@@ -661,7 +649,7 @@ __global__ void __launch_bounds__(256 * GROUPS, PER_SM)
   // alone for itself (the partials are a few tens of KB in L2), so the blocks
   // meet once a phase; of several films, a group each, and a second meeting.
   auto reduce = [&](uint32_t it, bool after_b) {
-    if (!blocks_meet(M, meet, polls, films, nfilms, step)) return false;
+    if (!blocks_meet(M, meet, polls)) return false;
     if (ONE) {
       if (threadIdx.z == 0) {
         const float total = group_total(only, after_b ? only.cg_part2 : only.cg_part, G.sv[0]);
@@ -690,7 +678,7 @@ __global__ void __launch_bounds__(256 * GROUPS, PER_SM)
         F.cg->beta = S.beta;
       }
     }
-    return blocks_meet(M, meet, polls, films, nfilms, step);
+    return blocks_meet(M, meet, polls);
   };
   // Walks the spans of the table, the tiles of one film at a time:
   // body(F, span, tx, ty) with the mask of the span's tiles that belong to F
@@ -728,6 +716,7 @@ __global__ void __launch_bounds__(256 * GROUPS, PER_SM)
     const float s = span_trees(G.sv, v);
     if (li < SPAN && ((on >> li) & 1u)) part[(uint32_t)tx + (uint32_t)ty * F.tw] = s;
   };
+  bool left_early = false;
   for (uint32_t it = 0; it < iters; ++it) {
     // p_it goes to cg_pa for even it, cg_pb for odd; p_{it-1} is in the other
     // (for it = 0 the init's direction, in cg_pa)
@@ -835,7 +824,10 @@ __global__ void __launch_bounds__(256 * GROUPS, PER_SM)
       }
       put_partials(F, F.cg_part, on, tx, ty, v);
     });
-    if (!reduce(it, false)) break;
+    if (!reduce(it, false)) {
+      left_early = true;
+      break;
+    }
     each_span(true, it, [&](const Film& F, uint32_t span, int tx, int ty) {
       const uint32_t fl = lane < SPAN && ((span >> lane) & 1u) ? F.tile_flags[(uint32_t)tx + (uint32_t)ty * F.tw] : 0u;
       const uint32_t on = __ballot_sync(0xffffffffu, (fl & ON) == ON);
@@ -870,8 +862,19 @@ __global__ void __launch_bounds__(256 * GROUPS, PER_SM)
       group_sync();  // the last span's sums have been read
       put_partials(F, F.cg_part2, on, tx, ty, v);
     });
-    if (!reduce(it, true)) break;
+    if (!reduce(it, true)) {
+      left_early = true;
+      break;
+    }
   }
+  // a wait ran out: every film that takes the step counts it and keeps its h
+  // through the step (kp_cg_finish)
+  if (left_early && lead_thread())
+    for (uint32_t f = first; f < nfilms; ++f)
+      if (step < films[f].P->implicit_steps) {
+        atomicAdd(&films[f].stats->wait_timeouts, 1u);
+        films[f].cg->failed = 1u;
+      }
   blocks_leave(M);
 }
 
